@@ -29,7 +29,7 @@ def build(with_reference=None):
     """make -C oracle [ref]; the reference part only where its sources exist."""
     subprocess.run(['make', '-s', '-C', str(HERE), 'all'], check=True)
     if with_reference is None:
-        with_reference = REFERENCE_ROOT.exists()
+        with_reference = any(REFERENCE_ROOT.glob('*'))  # an empty folder holds no sources
     if with_reference:
         subprocess.run(['make', '-s', '-C', str(HERE), 'ref', f'REF_ROOT={REFERENCE_ROOT}'], check=True)
 
