@@ -22,6 +22,12 @@ namespace bm25mlp {
 
 constexpr int kRows = 64;   // samples per forward CTA
 constexpr int kBRows = 32;  // samples per backward CTA
+constexpr int kBThreads = 256;
+constexpr int kBWarps = kBThreads / 32;
+constexpr int kTs = kBRows + 4;  // row strides in shared memory: a multiple of 16 bytes, and 8 lanes reading
+constexpr int kW2s = kH + 4;     // 16 bytes each from consecutive rows touch all 32 banks once
+static_assert(kH == 64 && kIn == 32 && kBRows == 32 && kBWarps * 4 == kBRows && kBWarps * 8 == kH,
+              "the backward kernel's thread tiles");
 
 __global__ void __launch_bounds__(kRows) ForwardKernel(const float *params, const float *x, long long batch, float *y)
 {
@@ -38,116 +44,257 @@ __global__ void __launch_bounds__(kRows) ForwardKernel(const float *params, cons
     y[r] = Forward(p, xi, h1, h2);
 }
 
-// Loss per sample: w * (y - t)^2 with w = over_weight when y > t (an over-estimate
-// of the K-th score sends the query to the plain path), else 1.  Mean over the batch.
-// Each CTA writes its partial gradient (kParams floats) and its loss sum.
-__global__ void __launch_bounds__(kBRows) BackwardKernel(const float *__restrict__ p, const float *x, const float *t,
-                                                         long long batch, float over_weight, float *partial,
-                                                         float *partial_loss)
+// acc[u][c] += sum over the row of w[unit lane + 32u][j] * in[j][4 * warp + c], j ascending.
+template <int kLen, int kStride>
+__device__ __forceinline__ void LayerTile(const float *w, const float *in, int lane, int warp, float (&acc)[2][4])
 {
-    __shared__ float sx[kBRows][kIn + 1];
-    __shared__ float sh1[kBRows][kH + 1], sd1[kBRows][kH + 1];
-    __shared__ float sh2[kBRows][kH + 1], sd2[kBRows][kH + 1];
-    __shared__ float sdy[kBRows], sloss[kBRows];
-    const int tid = threadIdx.x;
-    const long long r = (long long)blockIdx.x * kBRows + tid;
-    const bool live = r < batch;
-    float xi[kIn], h1[kH], h2[kH];
-    for (int j = 0; j < kIn; ++j)
-        xi[j] = live ? x[r * kIn + j] : 0.0f;
-    float dy = 0.0f, loss = 0.0f;
-    if (live) {
-        const float y = Forward(p, xi, h1, h2);
-        const float e = y - t[r];
-        const float w = e > 0.0f ? over_weight : 1.0f;
-        loss = w * e * e;
-        dy = 2.0f * w * e / (float)batch;
-    } else {
-        for (int i = 0; i < kH; ++i)
-            h1[i] = h2[i] = 0.0f;
-    }
-    // dh2 = dy * w3 (ReLU gate), dh1 = W2^T dh2 (ReLU gate)
-    float d2[kH];
-    for (int i = 0; i < kH; ++i)
-        d2[i] = h2[i] > 0.0f ? dy * p[kOffW3 + i] : 0.0f;
-    for (int j = 0; j < kH; ++j) {
-        float acc = 0.0f;
-        for (int i = 0; i < kH; ++i)
-            acc = fmaf(p[kOffW2 + i * kH + j], d2[i], acc);
-        sd1[tid][j] = h1[j] > 0.0f ? acc : 0.0f;
-        sh1[tid][j] = h1[j];
-        sh2[tid][j] = h2[j];
-        sd2[tid][j] = d2[j];
-    }
-    for (int j = 0; j < kIn; ++j)
-        sx[tid][j] = xi[j];
-    sdy[tid] = dy;
-    sloss[tid] = loss;
-    __syncthreads();
-    // this CTA's gradient, each parameter summed over the CTA's samples in row order
-    float *out = partial + (long long)blockIdx.x * kParams;
-    for (int q = tid; q < kParams; q += kBRows) {
-        float g = 0.0f;
-        if (q < kOffB1) {
-            const int i = (q - kOffW1) / kIn, j = (q - kOffW1) % kIn;
-            for (int s = 0; s < kBRows; ++s)
-                g = fmaf(sd1[s][i], sx[s][j], g);
-        } else if (q < kOffW2) {
-            const int i = q - kOffB1;
-            for (int s = 0; s < kBRows; ++s)
-                g += sd1[s][i];
-        } else if (q < kOffB2) {
-            const int i = (q - kOffW2) / kH, j = (q - kOffW2) % kH;
-            for (int s = 0; s < kBRows; ++s)
-                g = fmaf(sd2[s][i], sh1[s][j], g);
-        } else if (q < kOffW3) {
-            const int i = q - kOffB2;
-            for (int s = 0; s < kBRows; ++s)
-                g += sd2[s][i];
-        } else if (q < kOffB3) {
-            const int j = q - kOffW3;
-            for (int s = 0; s < kBRows; ++s)
-                g = fmaf(sdy[s], sh2[s][j], g);
-        } else {
-            for (int s = 0; s < kBRows; ++s)
-                g += sdy[s];
+#pragma unroll 4
+    for (int j = 0; j < kLen; j += 4) {
+        const float4 w0 = *reinterpret_cast<const float4 *>(w + lane * kStride + j);
+        const float4 w1 = *reinterpret_cast<const float4 *>(w + (lane + 32) * kStride + j);
+        const float wa[2][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}};
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            const float4 v = *reinterpret_cast<const float4 *>(in + (j + d) * kTs + 4 * warp);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                acc[u][0] = fmaf(wa[u][d], v.x, acc[u][0]);
+                acc[u][1] = fmaf(wa[u][d], v.y, acc[u][1]);
+                acc[u][2] = fmaf(wa[u][d], v.z, acc[u][2]);
+                acc[u][3] = fmaf(wa[u][d], v.w, acc[u][3]);
+            }
         }
-        out[q] = g;
-    }
-    if (tid == 0) {
-        float l = 0.0f;
-        for (int s = 0; s < kBRows; ++s)
-            l += sloss[s];
-        partial_loss[blockIdx.x] = l;
     }
 }
 
-// grad[q] = sum over CTAs of partial[c][q] in CTA order; loss = sum of partial losses / batch.
-__global__ void ReduceKernel(const float *partial, const float *partial_loss, int ctas, long long batch, float *grad,
-                             float *loss)
+// out[i][j] = sum over the CTA's samples, in row order, of d[i][s] * in[j][s]; warp w takes rows
+// 8w .. 8w + 7, lane l columns l, l + 32, ... (consecutive lanes write consecutive floats).
+template <int kCols> __device__ __forceinline__ void WeightGradient(const float *d, const float *in, int lane, int warp, float *out)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < kParams) {
+    constexpr int kN = kCols / 32;
+    float g[8][kN] = {};
+#pragma unroll 2
+    for (int s = 0; s < kBRows; s += 4) {
+        float4 v[kN];
+#pragma unroll
+        for (int n = 0; n < kN; ++n)
+            v[n] = *reinterpret_cast<const float4 *>(in + (lane + 32 * n) * kTs + s);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float4 e = *reinterpret_cast<const float4 *>(d + (8 * warp + r) * kTs + s);
+#pragma unroll
+            for (int n = 0; n < kN; ++n) {
+                g[r][n] = fmaf(e.x, v[n].x, g[r][n]);
+                g[r][n] = fmaf(e.y, v[n].y, g[r][n]);
+                g[r][n] = fmaf(e.z, v[n].z, g[r][n]);
+                g[r][n] = fmaf(e.w, v[n].w, g[r][n]);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int n = 0; n < kN; ++n)
+            out[(8 * warp + r) * kCols + lane + 32 * n] = g[r][n];
+}
+
+// Loss per sample: w * (y - t)^2 with w = over_weight when y > t (an over-estimate
+// of the K-th score sends the query to the plain path), else 1.  Mean over the batch.
+// Each CTA writes its partial gradient (kParams floats) and its loss sum.  Sample r is
+// row index[r] of x and t (index nullptr: row r).
+//
+// Bound: shared-memory loads and the FMA chains' latency, not HBM (a 4096-sample batch is 0.5 MB).
+// A thread owns units lane and lane + 32 of samples 4 * warp .. + 3 through all three layers, so a
+// 128-bit load of weights feeds 16 FMAs and one of activations 8; activations are kept [unit][sample],
+// which the layers read as broadcasts and the gradients along the samples.  Every sum is the chain
+// it would be with a thread per sample: index order, one accumulator.  Areas are reused as they die
+// (W1 -> h2 -> d2, W2 -> d1) to stay within the 48 KB that need no opt-in.  With a thread per sample,
+// its layers in local memory and one warp per CTA, 60 training steps of 4096 samples took 11.3 ms;
+// with this kernel and the batched sums below 4.3 ms, most of it the host's (same bits).
+__global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restrict__ p, const float *__restrict__ x,
+                                                            const float *__restrict__ t,
+                                                            const long long *__restrict__ index, long long batch,
+                                                            float over_weight, float *partial, float *partial_loss)
+{
+    __shared__ __align__(16) float sa[kH * kTs];   // W1 [unit][j], then h2, then d2 [unit][sample]
+    __shared__ __align__(16) float sw[kH * kW2s];  // W2 [unit][j], then d1 [unit][sample]
+    __shared__ __align__(16) float sx[kIn * kTs];  // x [j][sample]
+    __shared__ __align__(16) float sh1[kH * kTs];  // h1 [unit][sample]
+    __shared__ __align__(16) float sdy[kBRows];
+    __shared__ float sw3[kH], sloss[kBRows];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long r0 = (long long)blockIdx.x * kBRows;
+    float *out = partial + (long long)blockIdx.x * kParams;
+#pragma unroll
+    for (int i = 0; i < kBRows / kBWarps; ++i) {  // a warp reads one sample's row
+        const int s = warp * (kBRows / kBWarps) + i;
+        const long long r = r0 + s;
+        sx[lane * kTs + s] = r < batch ? x[(index ? index[r] : r) * kIn + lane] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < kH * kIn / kBThreads; ++i) {
+        const int q = tid + i * kBThreads;
+        sa[q / kIn * kTs + q % kIn] = p[kOffW1 + q];
+    }
+#pragma unroll
+    for (int i = 0; i < kH * kH / kBThreads; ++i) {
+        const int q = tid + i * kBThreads;
+        sw[q / kH * kW2s + q % kH] = p[kOffW2 + q];
+    }
+    if (tid < kH)
+        sw3[tid] = p[kOffW3 + tid];
+    float h1[2][4], h2[2][4];
+    bool live[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        live[c] = r0 + 4 * warp + c < batch;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            h1[u][c] = p[kOffB1 + lane + 32 * u];
+            h2[u][c] = p[kOffB2 + lane + 32 * u];
+        }
+    __syncthreads();
+    LayerTile<kIn, kTs>(sa, sx, lane, warp, h1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            h1[u][c] = live[c] ? fmaxf(h1[u][c], 0.0f) : 0.0f;
+        *reinterpret_cast<float4 *>(sh1 + (lane + 32 * u) * kTs + 4 * warp) =
+            make_float4(h1[u][0], h1[u][1], h1[u][2], h1[u][3]);
+    }
+    __syncthreads();
+    LayerTile<kH, kW2s>(sw, sh1, lane, warp, h2);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            h2[u][c] = live[c] ? fmaxf(h2[u][c], 0.0f) : 0.0f;
+        *reinterpret_cast<float4 *>(sa + (lane + 32 * u) * kTs + 4 * warp) =
+            make_float4(h2[u][0], h2[u][1], h2[u][2], h2[u][3]);
+    }
+    __syncthreads();
+    if (warp == 0) {  // the output of sample `lane`
+        const long long r = r0 + lane;
+        float dy = 0.0f, loss = 0.0f;
+        if (r < batch) {
+            float y = p[kOffB3];
+#pragma unroll 16
+            for (int j = 0; j < kH; ++j)
+                y = fmaf(sw3[j], sa[j * kTs + lane], y);
+            const float e = y - t[index ? index[r] : r];
+            const float w = e > 0.0f ? over_weight : 1.0f;
+            loss = w * e * e;
+            dy = 2.0f * w * e / (float)batch;
+        }
+        sdy[lane] = dy;
+        sloss[lane] = loss;
+    }
+    __syncthreads();
+    if (tid < kH) {  // w3's gradient, while h2 is there
         float g = 0.0f;
-        for (int c = 0; c < ctas; ++c)
-            g += partial[(long long)c * kParams + q];
-        grad[q] = g;
+#pragma unroll 8
+        for (int s = 0; s < kBRows; ++s)
+            g = fmaf(sdy[s], sa[tid * kTs + s], g);
+        out[kOffW3 + tid] = g;
+    } else if (tid == kH) {
+        float g = 0.0f, l = 0.0f;
+        for (int s = 0; s < kBRows; ++s) {
+            g += sdy[s];
+            l += sloss[s];
+        }
+        out[kOffB3] = g;
+        partial_loss[blockIdx.x] = l;
     }
-    if (q == 0 && loss) {
-        float l = 0.0f;
-        for (int c = 0; c < ctas; ++c)
-            l += partial_loss[c];
+    __syncthreads();
+    // dh2 = dy * w3 (ReLU gate), dh1 = W2^T dh2 (ReLU gate)
+    const float4 dy4 = *reinterpret_cast<const float4 *>(sdy + 4 * warp);
+    const float dy[4] = {dy4.x, dy4.y, dy4.z, dy4.w};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const float w3 = sw3[lane + 32 * u];
+        float d[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            d[c] = h2[u][c] > 0.0f ? dy[c] * w3 : 0.0f;
+        *reinterpret_cast<float4 *>(sa + (lane + 32 * u) * kTs + 4 * warp) = make_float4(d[0], d[1], d[2], d[3]);
+    }
+    __syncthreads();
+    float d1[2][4] = {};
+#pragma unroll 8
+    for (int i = 0; i < kH; ++i) {
+        const float4 v = *reinterpret_cast<const float4 *>(sa + i * kTs + 4 * warp);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const float w = sw[i * kW2s + lane + 32 * u];
+            d1[u][0] = fmaf(w, v.x, d1[u][0]);
+            d1[u][1] = fmaf(w, v.y, d1[u][1]);
+            d1[u][2] = fmaf(w, v.z, d1[u][2]);
+            d1[u][3] = fmaf(w, v.w, d1[u][3]);
+        }
+    }
+    WeightGradient<kH>(sa, sh1, lane, warp, out + kOffW2);
+    __syncthreads();  // W2 has been read by every warp
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            d1[u][c] = h1[u][c] > 0.0f ? d1[u][c] : 0.0f;
+        *reinterpret_cast<float4 *>(sw + (lane + 32 * u) * kTs + 4 * warp) =
+            make_float4(d1[u][0], d1[u][1], d1[u][2], d1[u][3]);
+    }
+    __syncthreads();
+    WeightGradient<kIn>(sw, sx, lane, warp, out + kOffW1);
+    if (tid < 2 * kH) {  // the biases' gradients
+        const float *d = (tid < kH ? sw : sa) + tid % kH * kTs;
+        float g = 0.0f;
+#pragma unroll 8
+        for (int s = 0; s < kBRows; ++s)
+            g += d[s];
+        out[(tid < kH ? kOffB1 : kOffB2) + tid % kH] = g;
+    }
+}
+
+constexpr int kReduceThreads = 64;  // 100 CTAs: each thread's chain of loads is what takes the time
+
+// Sum of partial[c][q] in CTA order (32 loads in flight, one accumulator).
+__device__ __forceinline__ float SumPartials(const float *__restrict__ partial, int q, int ctas)
+{
+    float g = 0.0f;
+    int c = 0;
+    for (; c + 32 <= ctas; c += 32) {
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            v[i] = partial[(long long)(c + i) * kParams + q];
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            g += v[i];
+    }
+    for (; c < ctas; ++c)
+        g += partial[(long long)c * kParams + q];
+    return g;
+}
+
+// The batch's mean loss: one warp loads, the sum is in CTA order.
+__device__ __forceinline__ void BatchLoss(const float *__restrict__ partial_loss, int ctas, long long batch, int lane,
+                                          float *loss)
+{
+    float l = 0.0f;
+    for (int c = 0; c < ctas; c += 32) {
+        const float v = c + lane < ctas ? partial_loss[c + lane] : 0.0f;
+        for (int i = 0; i < min(32, ctas - c); ++i)
+            l += __shfl_sync(0xffffffffu, v, i);
+    }
+    if (lane == 0)
         *loss = l / (float)batch;
-    }
 }
 
 // Adam (beta1 0.9, beta2 0.999, eps 1e-8) with bias correction for step `step` (1-based).
-__global__ void AdamKernel(float *params, float *m, float *v, const float *grad, float lr, int step)
+__device__ __forceinline__ void AdamUpdate(float *params, float *m, float *v, float g, float lr, int step, int q)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= kParams)
-        return;
-    const float g = grad[q];
     const float mq = 0.9f * m[q] + 0.1f * g, vq = 0.999f * v[q] + 0.001f * g * g;
     m[q] = mq;
     v[q] = vq;
@@ -155,9 +302,32 @@ __global__ void AdamKernel(float *params, float *m, float *v, const float *grad,
     params[q] -= lr * mh / (sqrtf(vh) + 1e-8f);
 }
 
+// grad[q] = sum over CTAs of partial[c][q] in CTA order; loss = sum of partial losses / batch.
+// The loss is the last CTA's, which has no parameters.
+__global__ void __launch_bounds__(kReduceThreads) ReduceKernel(const float *partial, const float *partial_loss, int ctas,
+                                                               long long batch, float *grad, float *loss)
+{
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x < 32 && loss)
+            BatchLoss(partial_loss, ctas, batch, threadIdx.x, loss);
+        return;
+    }
+    const int q = blockIdx.x * kReduceThreads + threadIdx.x;
+    if (q < kParams)
+        grad[q] = SumPartials(partial, q, ctas);
+}
+
+__global__ void AdamKernel(float *params, float *m, float *v, const float *grad, float lr, int step)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < kParams)
+        AdamUpdate(params, m, v, grad[q], lr, step, q);
+}
+
 } // namespace bm25mlp
 
 namespace {
+constexpr int kReduceCtas = (bm25mlp::kParams + bm25mlp::kReduceThreads - 1) / bm25mlp::kReduceThreads;
 thread_local std::string g_mlp_error;
 int Fail(int status, const std::string &m)
 {
@@ -200,13 +370,13 @@ extern "C" int bm25_mlp_gradient(const float *params, const float *features, con
         return Fail(BM25_ERR_INVALID_PARAM, "Batch too large");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     float *partial = scratch, *partial_loss = scratch + ctas * bm25mlp::kParams;
-    bm25mlp::BackwardKernel<<<(unsigned)ctas, bm25mlp::kBRows, 0, s>>>(params, features, targets, batch, over_weight,
-                                                                      partial, partial_loss);
+    bm25mlp::BackwardKernel<<<(unsigned)ctas, bm25mlp::kBThreads, 0, s>>>(params, features, targets, nullptr, batch,
+                                                                         over_weight, partial, partial_loss);
     int st = CudaStatus(cudaGetLastError(), "MLP backward launch");
     if (st != BM25_OK)
         return st;
-    bm25mlp::ReduceKernel<<<(bm25mlp::kParams + 255) / 256, 256, 0, s>>>(partial, partial_loss, (int)ctas, batch,
-                                                                          grad, loss);
+    bm25mlp::ReduceKernel<<<kReduceCtas + 1, bm25mlp::kReduceThreads, 0, s>>>(partial, partial_loss, (int)ctas, batch,
+                                                                              grad, loss);
     return CudaStatus(cudaGetLastError(), "MLP reduce launch");
 }
 

@@ -88,3 +88,24 @@ def test_adam_training_fits_a_smooth_target(pkg, cuda_ok):
     torch.cuda.synchronize()
     final = mo.loss(dp.cpu().numpy(), x, t, 1.0)
     assert final < 0.2 * first, (first, final)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('batch', [1, 31, 32, 33, 1023, 1025, 4097])  # the row block, and 32 blocks' sums at a time
+def test_gradient_at_row_block_edges(pkg, cuda_ok, batch):
+    import torch
+    lib = pkg._native.engine_library()
+    rng = np.random.default_rng(batch)
+    p = mo.init(5)
+    x = rng.normal(size=(batch, mo.IN)).astype(np.float32)
+    t = rng.normal(size=batch).astype(np.float32)
+    dp, dx, dt = _dev(torch, p), _dev(torch, x), _dev(torch, t)
+    scratch = torch.full((lib.bm25_mlp_scratch_floats(batch),), float('nan'), dtype=torch.float32, device='cuda')
+    g = torch.empty(mo.PARAMS, dtype=torch.float32, device='cuda')
+    loss = torch.empty(1, dtype=torch.float32, device='cuda')
+    assert lib.bm25_mlp_gradient(dp.data_ptr(), dx.data_ptr(), dt.data_ptr(), batch, ctypes.c_float(4.0),
+                                 scratch.data_ptr(), g.data_ptr(), loss.data_ptr(), None) == 0
+    # FP32 chains of at most 64 + 32 + batch / 32 terms: 1e-4 of the largest entry covers their rounding
+    gref = mo.gradient(p, x, t, 4.0)
+    assert np.abs(g.cpu().numpy() - gref).max() <= 1e-4 * np.abs(gref).max()
+    assert abs(loss.item() - mo.loss(p, x, t, 4.0)) <= 1e-4 * mo.loss(p, x, t, 4.0)
