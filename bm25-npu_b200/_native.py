@@ -150,6 +150,8 @@ SIGNATURES = {
     'bm25_mlp_gradient': (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_float, c_void_p, c_void_p, c_void_p,
                                   c_void_p]),
     'bm25_mlp_adam': (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int32, c_void_p]),
+    'bm25_mlp_train_steps': (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32,
+                                     c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p]),
     'bm25_mlp_last_error': (c_int, [ctypes.c_char_p, c_size_t]),
     'bm25_search_csc_static': (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64,
                                        c_int64, c_int32, c_void_p, c_void_p, c_void_p, c_int32]),

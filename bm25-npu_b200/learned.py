@@ -23,6 +23,7 @@ from . import _native as n
 
 FEATURES = 32
 HIDDEN = 64
+_TRAIN_STEPS = 8  # steps whose row numbers are drawn and copied at once, while the steps before them run
 
 
 def param_count():
@@ -109,26 +110,21 @@ def train(features, targets, *, steps=3000, batch=4096, lr=2e-3, over_weight=4.0
     t = torch.from_numpy(np.ascontiguousarray(targets, dtype=np.float32)).to(dev)
     count = x.shape[0]
     batch = min(batch, count)
+    if x.numel() != count * FEATURES or t.numel() != t.shape[0] or t.shape[0] < count:
+        raise ValueError('train: features [N, 32] and one target per row expected')
     p = torch.from_numpy(init_params(seed, float(np.mean(targets)))).to(dev)
     m = torch.zeros_like(p)
     v = torch.zeros_like(p)
-    g = torch.zeros_like(p)
     loss = torch.zeros(steps, dtype=torch.float32, device=dev)
     scratch = torch.empty(int(lib.bm25_mlp_scratch_floats(batch)), dtype=torch.float32, device=dev)
-    xb = torch.empty((batch, FEATURES), dtype=torch.float32, device=dev)
-    tb = torch.empty(batch, dtype=torch.float32, device=dev)
     rng = np.random.default_rng(seed + 1)
     stream = torch.cuda.current_stream(dev).cuda_stream
-    for step in range(steps):
-        idx = torch.from_numpy(rng.integers(0, count, batch)).to(dev)
-        torch.index_select(x, 0, idx, out=xb)
-        torch.index_select(t, 0, idx, out=tb)
-        _check(lib.bm25_mlp_gradient(c_void_p(p.data_ptr()), c_void_p(xb.data_ptr()), c_void_p(tb.data_ptr()), batch,
-                                     c_float(over_weight), c_void_p(scratch.data_ptr()), c_void_p(g.data_ptr()),
-                                     c_void_p(loss[step:].data_ptr()), c_void_p(stream)), 'MLP gradient')
-        _check(lib.bm25_mlp_adam(c_void_p(p.data_ptr()), c_void_p(m.data_ptr()), c_void_p(v.data_ptr()),
-                                 c_void_p(g.data_ptr()), c_float(lr), c_int32(step + 1), c_void_p(stream)),
-               'MLP Adam')
+    for step in range(0, steps, _TRAIN_STEPS):
+        rows = rng.integers(0, count, (min(_TRAIN_STEPS, steps - step), batch))
+        index = torch.from_numpy(rows).to(dev)
+        _check(lib.bm25_mlp_train_steps(p.data_ptr(), m.data_ptr(), v.data_ptr(), x.data_ptr(), t.data_ptr(),
+                                        index.data_ptr(), batch, len(rows), step + 1, over_weight, lr,
+                                        scratch.data_ptr(), loss[step:].data_ptr(), stream), 'MLP training')
     torch.cuda.synchronize(dev)
     return p.cpu().numpy(), loss.cpu().numpy()
 

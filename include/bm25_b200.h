@@ -328,6 +328,10 @@ int bm25_kernel_times(bm25_handle *h, float *ms, int64_t capacity, int64_t *coun
  *     and *loss = that mean; deterministic (fixed summation order).  `scratch`
  *     holds bm25_mlp_scratch_floats(batch) floats.  `loss` may be NULL.
  *   bm25_mlp_adam: one Adam step (beta1 0.9, beta2 0.999, eps 1e-8), step >= 1.
+ *   bm25_mlp_train_steps: `steps` gradient and Adam steps from step number
+ *     first_step; step i's samples are rows rows[i * batch ..] (int64, each inside
+ *     the arrays) of features and targets, its loss goes to loss[i].  The results
+ *     are those of the two calls above on the gathered samples.
  * Error details: bm25_mlp_last_error.
  */
 int64_t bm25_mlp_param_count(void);
@@ -336,6 +340,9 @@ int bm25_mlp_forward(const float *params, const float *features, int64_t batch, 
 int bm25_mlp_gradient(const float *params, const float *features, const float *targets, int64_t batch,
                       float over_weight, float *scratch, float *grad, float *loss, void *stream);
 int bm25_mlp_adam(float *params, float *m, float *v, const float *grad, float lr, int32_t step, void *stream);
+int bm25_mlp_train_steps(float *params, float *m, float *v, const float *features, const float *targets,
+                         const int64_t *rows, int64_t batch, int32_t steps, int32_t first_step, float over_weight,
+                         float lr, float *scratch, float *loss, void *stream);
 int bm25_mlp_last_error(char *buffer, size_t length);
 
 /*

@@ -109,3 +109,31 @@ def test_gradient_at_row_block_edges(pkg, cuda_ok, batch):
     gref = mo.gradient(p, x, t, 4.0)
     assert np.abs(g.cpu().numpy() - gref).max() <= 1e-4 * np.abs(gref).max()
     assert abs(loss.item() - mo.loss(p, x, t, 4.0)) <= 1e-4 * mo.loss(p, x, t, 4.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('batch', [1, 33, 1025])
+def test_train_steps_are_gradient_and_adam_on_the_gathered_rows(pkg, cuda_ok, batch):
+    import torch
+    lib = pkg._native.engine_library()
+    rng = np.random.default_rng(batch)
+    x, t = _dev(torch, rng.normal(size=(2000, mo.IN))), _dev(torch, rng.normal(size=2000))
+    rows = torch.from_numpy(rng.integers(0, 2000, (5, batch))).cuda()
+    scratch = torch.empty(lib.bm25_mlp_scratch_floats(batch), dtype=torch.float32, device='cuda')
+    want = [_dev(torch, mo.init(9)), torch.zeros(mo.PARAMS, device='cuda'), torch.zeros(mo.PARAMS, device='cuda')]
+    got = [a.clone() for a in want]
+    g, loss, losses = torch.empty(mo.PARAMS, device='cuda'), torch.empty(5, device='cuda'), torch.empty(5, device='cuda')
+    for i in range(5):
+        xb, tb = x[rows[i]].contiguous(), t[rows[i]].contiguous()
+        assert lib.bm25_mlp_gradient(want[0].data_ptr(), xb.data_ptr(), tb.data_ptr(), batch, ctypes.c_float(4.0),
+                                     scratch.data_ptr(), g.data_ptr(), loss[i:].data_ptr(), None) == 0
+        assert lib.bm25_mlp_adam(want[0].data_ptr(), want[1].data_ptr(), want[2].data_ptr(), g.data_ptr(),
+                                 ctypes.c_float(2e-3), i + 1, None) == 0
+        torch.cuda.synchronize()
+    for first in (0, 2):  # in two calls
+        n = 2 if first == 0 else 3
+        assert lib.bm25_mlp_train_steps(got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr(), x.data_ptr(),
+                                        t.data_ptr(), rows[first:].data_ptr(), batch, n, first + 1, 4.0, 2e-3,
+                                        scratch.data_ptr(), losses[first:].data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got + [losses], want + [loss]))
