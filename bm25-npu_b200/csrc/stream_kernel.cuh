@@ -161,6 +161,7 @@ struct StreamArgs {
     int *plan_rows;
     int4 *word_rec;
     int rows_plan;
+    int seed_threshold;  // PlanRowsKernel raises the queries' thresholds to their words' seeds
     int prefetch;
     // [vocab][32] each term's 32 largest posting scores (descending, 0 past its document
     // frequency): the warp-tile kernel starts a K <= 32 query's running bound at the largest K-th

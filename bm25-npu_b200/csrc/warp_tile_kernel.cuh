@@ -447,7 +447,8 @@ inline const void *WarpTileKernelFor(bool lean)
 // The CTAs of chunk 0 also write each word's record: its seed -- the word's posting score at rank
 // K of its query (term_top for K <= 32, else the smallest stored rank 64, 128, ..., 1024 not
 // below K), which K documents reach (0 without term statistics) --, its dense row, and its
-// directory row (-1: a short list; -2: not a term).  One CTA also empties the block path's work
+// directory row (-1: a short list; -2: not a term) -- and, for a first pass of the tile-group kernel
+// (seed_threshold), raise the query's threshold to the seed.  One CTA also empties the block path's work
 // lists of the Search (when it has them), as PlanKernel does where it runs.
 __global__ void __launch_bounds__(kPlanThreads) PlanRowsKernel(const StreamArgs a)
 {
@@ -476,11 +477,11 @@ __global__ void __launch_bounds__(kPlanThreads) PlanRowsKernel(const StreamArgs 
         const int term = __ldg(a.words + w);
         int *out = a.plan_rows + w * a.dir_stride;
         const bool known = term >= 0 && term < a.vocab;
-        // a K per query: the word's query is the number of q in [1, Q] with qoffsets[q] <= w (the last
+        // a K per query, or a threshold to seed: the word's query is the number of q in [1, Q] with qoffsets[q] <= w (the last
         // query starting at or before w), counted by the whole CTA at once (a malformed batch is
         // flagged by the search kernel and fails as a whole)
         int wq = 0;
-        if (a.kq && blockIdx.y == 0) {  // uniform
+        if ((a.kq || a.seed_threshold) && blockIdx.y == 0) {  // uniform
             for (int base = 1; base <= a.q; base += kPlanThreads)
                 wq += __syncthreads_count(base + tid <= a.q && __ldg(a.qoffsets + base + tid) <= w);
             wq = min(wq, a.q - 1);
@@ -501,6 +502,8 @@ __global__ void __launch_bounds__(kPlanThreads) PlanRowsKernel(const StreamArgs 
                 atomicOr(a.status, kStatusBadWord);
             }
             a.word_rec[w] = make_int4(__float_as_int(seed), drow, dr, 0);
+            if (a.seed_threshold && seed > 0.0f)
+                atomicMax(a.threshold + wq, __float_as_uint(seed));  // positive floats order as their bits
         }
         if (!known) {  // no postings
             for (int t = e0 + tid; t < e1; t += kPlanThreads)

@@ -160,3 +160,30 @@ def test_tune_batch_with_k_per_query_learned(pkg, oracle_mod, corpus, cuda_ok):
         assert len(table) == 2 and best['prune_route'] in (0.2, 1.0) and s.tuning()['prune_route'] == best['prune_route']
         got_s, got_i, _, _ = s.search_batch((offsets, words), ks, learned=True)
         assert_same_topk(got_s[None], got_i[None], want_s[None], want_i[None], 'tuned learned batch')
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('k', [33, 64, 65, 1000, 1024])
+def test_large_k_from_seeds_with_ties(pkg, oracle_mod, cuda_ok, k):
+    """Words whose seed (the score at a stored rank) equals the K-th score, with ties past it, lists of
+    exactly K and K - 1 postings, and scores over many octaves; one K and a K per query."""
+    rng = np.random.default_rng(k)
+    docs = 50_001
+    lists = [(docs // 2, 1.0), (k, 2.0), (k - 1, 3.0), (2048, None), (1, 4.0)]
+    ids = [np.sort(rng.choice(docs, size=n, replace=False)).astype(np.int32) for n, _ in lists]
+    data = [np.full(n, v, np.float32) if v else np.exp2(rng.uniform(-20, 20, n)).astype(np.float32) for n, v in lists]
+    indptr = np.concatenate([[0], np.cumsum([n for n, _ in lists])]).astype(np.int64)
+    ids, data = np.concatenate(ids), np.concatenate(data)
+    offsets, words = pack([[0], [1], [2], [3], [0, 1], [2, 3, 0], [], [4, 1], [3, 3], [4]])
+    want = oracle_mod.search(indptr, ids, data, docs, offsets, words, k)
+    with pkg.Bm25Session.from_csc(indptr, ids, data, docs, query_capacity=16, word_capacity=64, max_k=1024) as s:
+        for _ in range(2):
+            assert_same_topk(*s.search((offsets, words), k), *want, f'k={k}')
+        ks = np.resize(np.array([k, 10, 32], np.int32), offsets.size - 1)
+        scores, got, _ = s.search_batch((offsets, words), ks)
+        start = 0
+        for q, kq in enumerate(ks):
+            ref = oracle_mod.search(indptr, ids, data, docs, *pack([words[offsets[q]:offsets[q + 1]].tolist()]), int(kq))
+            assert_same_topk(scores[start:start + kq], got[start:start + kq], ref[0].ravel(), ref[1].ravel(), f'q={q}')
+            start += kq
+        assert s.device_status() == 0
