@@ -1302,15 +1302,17 @@ class Engine {
                 sa.item_count = d_item_count_;
                 sa.item_cap = item_cap_;
             }
-            // A warp-tile session runs the warp-tile kernel for plain Searches of one K <= 32 and for
-            // every pass that streams from a bound already set (the routed queries of a pruned Search,
-            // from their learned bound; retry passes, from their proven one), all on the plan rows of
-            // the Search's words.  The first pass of a pruned Search is block-scored (block-tile
-            // kernel, also on the plan rows); that of a batch with a K per query or K > 32 runs the
-            // tile-group kernel on the (query word, tile) plan (the warp-tile kernel's wider first
-            // wave of claims would append far more candidates there).
+            // A warp-tile session runs the warp-tile kernel for plain Searches of K <= 32 (one K, or a K
+            // per query) and for every pass that streams from a bound already set (the routed queries of
+            // a pruned Search, from their learned bound; retry passes, from their proven one), all on the
+            // plan rows of the Search's words.  The first pass of a pruned Search is block-scored
+            // (block-tile kernel, also on the plan rows); that of a batch whose largest K is above 32 runs
+            // the tile-group kernel on the (query word, tile) plan: its bound rises late, and the warp-tile
+            // kernel's wider first wave of claims appends far more candidates.  Tile-group against
+            // warp-tile kernel, us a Search: 50 queries at K 10 and 32 on 262,147 documents 99 / 90 to 97; 37 at
+            // K 1000 on 1M 434 / 477; 256 at K 10, 100 and 1000 on 8.8M 6180 / 7542.
             const bool wt_session = plan_.kernel == BM25_KERNEL_WARP_TILE;
-            const bool warp_tile = wt_session && !tau && !kq && k <= bm25k::kMaxSmallK;
+            const bool warp_tile = wt_session && !tau && k <= bm25k::kMaxSmallK;
             // the streaming passes after a first pass (retries, routed queries) run the warp-tile kernel
             // too, on the plan rows; a pruned Search of a warp-tile session takes its block path's
             // ranges from the plan rows as well and builds no (query word, tile) plan
@@ -1321,7 +1323,7 @@ class Engine {
             // bound): otherwise every claim taken before the first tiles are selected appends all it has
             // (37 queries at K 1000 on 1M documents: 643 -> 434 us a Search; 256 mixed queries on 8.8M:
             // 7.2 -> 6.2 ms; 50 queries at K 10 and 32 on 262,147: 156 -> 99 us)
-            sa.seed_threshold = wt_session && !tau && !warp_tile ? 1 : 0;
+            sa.seed_threshold = wt_session && !tau && (kq || !warp_tile) ? 1 : 0;
             sa.plan_rows = plan_rows_;
             sa.word_rec = word_rec_;
             sa.prefetch = 1;
