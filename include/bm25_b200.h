@@ -81,8 +81,8 @@ typedef struct bm25_options {
  *   BM25_KERNEL_WARP_TILE  persistent kernel, 1024-document tiles, every warp takes its own claims
  *                          (a query and 4 consecutive tiles) and loads its postings itself, the
  *                          claim's posting runs prefetched into L2 (the default) -- for plain
- *                          Searches with one K <= 32; pruned Searches, batches with a K per query
- *                          and K > 32 run the tile-group kernel */
+ *                          Searches with K <= 32 (one K, or a K per query); K > 32 runs the
+ *                          tile-group kernel, pruned Searches the block path */
 #define BM25_KERNEL_STREAM 0
 #define BM25_KERNEL_PER_TILE 1
 #define BM25_KERNEL_TILE_GROUP 4
