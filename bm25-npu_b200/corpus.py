@@ -205,5 +205,6 @@ def build_index(doc_offsets, tokens, vocab, k1=1.2, b=0.75, device_id=0):
         lib.bm25_build_last_error(buf, len(buf))
         raise ValueError(f'index build failed ({status}): {buf.value.decode()}')
     k = m.value
-    return LazyIndex(offsets, docs[:k].copy(), tf[:k].copy(), norm, idf,
+    # the arrays are as long as the tokens; the pages past the postings were never touched
+    return LazyIndex(offsets, docs[:k], tf[:k], norm, idf,
                      np.diff(doc_offsets).astype(np.int32))

