@@ -116,7 +116,9 @@ template <int kCols> __device__ __forceinline__ void WeightGradient(const float 
 // (W1 -> h2 -> d2, W2 -> d1) to stay within the 48 KB that need no opt-in.  With a thread per sample,
 // its layers in local memory and one warp per CTA, 60 training steps of 4096 samples took 11.3 ms;
 // with this kernel and the batched sums below 4.3 ms, most of it the host's (same bits).
-__global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restrict__ p, const float *__restrict__ x,
+// In a training loop this kernel starts while the update before it still writes p: p makes no promise
+// of being constant, and is read after the wait, from L2 (x, t and index are constant).
+__global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *p, const float *__restrict__ x,
                                                             const float *__restrict__ t,
                                                             const long long *__restrict__ index, long long batch,
                                                             float over_weight, float *partial, float *partial_loss)
@@ -141,15 +143,15 @@ __global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restr
 #pragma unroll
     for (int i = 0; i < kH * kIn / kBThreads; ++i) {
         const int q = tid + i * kBThreads;
-        sa[q / kIn * kTs + q % kIn] = p[kOffW1 + q];
+        sa[q / kIn * kTs + q % kIn] = __ldcg(p + kOffW1 + q);
     }
 #pragma unroll
     for (int i = 0; i < kH * kH / kBThreads; ++i) {
         const int q = tid + i * kBThreads;
-        sw[q / kH * kW2s + q % kH] = p[kOffW2 + q];
+        sw[q / kH * kW2s + q % kH] = __ldcg(p + kOffW2 + q);
     }
     if (tid < kH)
-        sw3[tid] = p[kOffW3 + tid];
+        sw3[tid] = __ldcg(p + kOffW3 + tid);
     float h1[2][4], h2[2][4];
     bool live[4];
 #pragma unroll
@@ -159,8 +161,8 @@ __global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restr
     for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            h1[u][c] = p[kOffB1 + lane + 32 * u];
-            h2[u][c] = p[kOffB2 + lane + 32 * u];
+            h1[u][c] = __ldcg(p + kOffB1 + lane + 32 * u);
+            h2[u][c] = __ldcg(p + kOffB2 + lane + 32 * u);
         }
     __syncthreads();
     LayerTile<kIn, kTs>(sa, sx, lane, warp, h1);
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kBThreads) BackwardKernel(const float *__restr
         const long long r = r0 + lane;
         float dy = 0.0f, loss = 0.0f;
         if (r < batch) {
-            float y = p[kOffB3];
+            float y = __ldcg(p + kOffB3);
 #pragma unroll 16
             for (int j = 0; j < kH; ++j)
                 y = fmaf(sw3[j], sa[j * kTs + lane], y);

@@ -1,6 +1,8 @@
 """Threshold MLP: the CUDA forward/backward/Adam kernels against the float64 CPU oracle."""
 
 import ctypes
+import re
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -135,5 +137,47 @@ def test_train_steps_are_gradient_and_adam_on_the_gathered_rows(pkg, cuda_ok, ba
         assert lib.bm25_mlp_train_steps(got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr(), x.data_ptr(),
                                         t.data_ptr(), rows[first:].data_ptr(), batch, n, first + 1, 4.0, 2e-3,
                                         scratch.data_ptr(), losses[first:].data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got + [losses], want + [loss]))
+
+
+def test_overlapped_backward_makes_no_promise_of_constant_parameters():
+    """A training step's backward kernel starts while the update before it writes the parameters: a
+    __restrict__ const argument or a read-only load of them may be moved above the wait."""
+    src = (Path(__file__).resolve().parents[1] / 'bm25-npu_b200' / 'csrc' / 'mlp.cu').read_text()
+    kernel = re.search(r'BackwardKernel\(const float \*.*?\n}\n', src, re.S).group()
+    signature, body = kernel.split('{', 1)
+    assert re.match(r'BackwardKernel\(const float \*p,', signature), signature
+    before, after = body.split('WaitPrerequisites();')
+    assert not re.search(r'\bp\b', before)  # nothing of p is read before the wait
+    assert not re.search(r'\bp\[|__ldg\(p\b', after) and after.count('__ldcg(p + ') == 6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('batch', [4096, 4097])  # 128 and 129 CTAs: the backward kernel on nearly every SM
+def test_overlapped_training_steps_see_each_update(pkg, cuda_ok, batch):
+    """Twelve overlapped steps in one call have the bits of separate gradient and Adam calls."""
+    import torch
+    lib = pkg._native.engine_library()
+    steps = 12
+    rng = np.random.default_rng(batch)
+    x, t = _dev(torch, rng.normal(size=(9000, mo.IN))), _dev(torch, rng.normal(size=9000))
+    rows = torch.from_numpy(rng.integers(0, 9000, (steps, batch))).cuda()
+    scratch = torch.empty(lib.bm25_mlp_scratch_floats(batch), dtype=torch.float32, device='cuda')
+    want = [_dev(torch, mo.init(9)), torch.zeros(mo.PARAMS, device='cuda'), torch.zeros(mo.PARAMS, device='cuda')]
+    got = [a.clone() for a in want]
+    g = torch.empty(mo.PARAMS, device='cuda')
+    loss, losses = torch.empty(steps, device='cuda'), torch.empty(steps, device='cuda')
+    for i in range(steps):
+        xb, tb = x[rows[i]].contiguous(), t[rows[i]].contiguous()
+        torch.cuda.synchronize()
+        assert lib.bm25_mlp_gradient(want[0].data_ptr(), xb.data_ptr(), tb.data_ptr(), batch, ctypes.c_float(4.0),
+                                     scratch.data_ptr(), g.data_ptr(), loss[i:].data_ptr(), None) == 0
+        assert lib.bm25_mlp_adam(want[0].data_ptr(), want[1].data_ptr(), want[2].data_ptr(), g.data_ptr(),
+                                 ctypes.c_float(2e-3), i + 1, None) == 0
+        torch.cuda.synchronize()
+    assert lib.bm25_mlp_train_steps(got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr(), x.data_ptr(),
+                                    t.data_ptr(), rows.data_ptr(), batch, steps, 1, 4.0, 2e-3, scratch.data_ptr(),
+                                    losses.data_ptr(), None) == 0
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got + [losses], want + [loss]))
