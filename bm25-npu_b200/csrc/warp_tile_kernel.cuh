@@ -290,6 +290,11 @@ __global__ void __launch_bounds__(kWtThreads, 3) WarpTileKernel(const StreamArgs
             bad |= kStatusBadQuery;
             nw = 0;
         }
+        if (nw == 0) {  // uniform: nothing to scan (a batch is padded to its bucket with empty queries)
+            if (lane == 0)
+                sh.counters[warp][0] += 1u;
+            continue;
+        }
         const int k = kLean ? a.k : QueryK(a, q);
         int offA[kC + 1];  // word `lane`'s posting positions at the claim's tile bounds
 #pragma unroll

@@ -106,3 +106,17 @@ def test_batch_buckets_pad_exactly(pkg, oracle_mod, corpus, cuda_ok):
             qo, w = pkg.synthetic_queries(index.offsets, q, 1, 4, q)
             s.search_batch((qo, w), np.full(q, 100, np.int32))
         assert s.info()['graph_instantiations'] == made
+
+
+@pytest.mark.gpu
+def test_padding_of_a_batch_scans_no_tiles(pkg, corpus, cuda_ok):
+    """A batch padded to its bucket (5 of 8, K <= 32) scans the tiles of its queries with words alone."""
+    index, data = corpus
+    tiles = -(-index.num_docs // 1024)
+    qo, w = pkg.synthetic_queries(index.offsets, 4, 2, 4, 5)
+    qo = np.insert(qo, 2, qo[2])  # and one empty query among them
+    with pkg.Bm25Session.from_csc(index.offsets, index.docs, data, index.num_docs, query_capacity=16,
+                                  word_capacity=64, max_k=32) as s:
+        s.search_stats(reset=True)
+        s.search_batch((qo, w), np.array([10, 32, 1, 10, 32], np.int32))
+        assert s.search_stats(reset=True)['tiles_scanned'] == 4 * tiles
