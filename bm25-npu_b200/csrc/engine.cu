@@ -1356,9 +1356,13 @@ class Engine {
             const long long claims = (long long)q * ((plan_.tiles + bm25k::kWgWarps - 1) / bm25k::kWgWarps);
             const int wg_grid = (int)std::max<long long>(1, std::min<long long>(tg_grid_, claims));
             const int ct = tuning_.claim_tiles;
-            const long long wt_claims = (long long)q * ((plan_.tiles + ct - 1) / ct);
+            // one warp per tile while the chip has them (the claims below are then all single tiles): a grid
+            // of one warp per claim of ct tiles left most SMs idle and a chain of tiles to each warp on
+            // small work, where a batch of K <= 32 took longer than on the tile-group kernel (1 query on
+            // 262,147 documents 62 us against 60, 256 on 8192 162 against 147; 57 and 140 with this grid)
+            const long long wt_tiles = (long long)q * plan_.tiles;
             const int wt_grid = (int)std::max<long long>(
-                1, std::min<long long>(plan_.grid, (wt_claims + bm25k::kWtWarps - 1) / bm25k::kWtWarps));
+                1, std::min<long long>(plan_.grid, (wt_tiles + bm25k::kWtWarps - 1) / bm25k::kWtWarps));
             {
                 // single-tile claims for the last tiles: tail_claims per warp of the launch
                 const long long tail = ((long long)tuning_.tail_claims * wt_grid * bm25k::kWtWarps + q - 1) / q;

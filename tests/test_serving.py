@@ -120,3 +120,24 @@ def test_padding_of_a_batch_scans_no_tiles(pkg, corpus, cuda_ok):
         s.search_stats(reset=True)
         s.search_batch((qo, w), np.array([10, 32, 1, 10, 32], np.int32))
         assert s.search_stats(reset=True)['tiles_scanned'] == 4 * tiles
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('q', [1, 8])
+def test_small_batch_gives_each_tile_its_own_warp(pkg, oracle_mod, corpus, cuda_ok, q):
+    """Fewer tiles than the chip has warps (98 a query here): every claim is a single tile, and the rows
+    are the oracle's."""
+    index, data = corpus
+    tiles = -(-index.num_docs // 1024)
+    qo, w = pkg.synthetic_queries(index.offsets, q, 2, 4, 5)
+    ks = np.resize(np.array([10, 32], np.int32), q)
+    with pkg.Bm25Session.from_csc(index.offsets, index.docs, data, index.num_docs, query_capacity=8,
+                                  word_capacity=64, max_k=32) as s:
+        s.search_stats(reset=True)
+        gs, gi, koff = s.search_batch((qo, w), ks)
+        assert s.search_stats(reset=True)['claims'] == q * tiles
+    for i in range(q):
+        want = oracle_mod.search(index.offsets, index.docs, data, index.num_docs, qo[i:i + 2] - qo[i],
+                                 w[qo[i]:qo[i + 1]], int(ks[i]))
+        assert np.array_equal(gi[koff[i]:koff[i + 1]], want[1][0])
+        assert np.array_equal(gs[koff[i]:koff[i + 1]].view(np.uint32), want[0][0].view(np.uint32))
