@@ -1193,8 +1193,9 @@ __global__ void __launch_bounds__(kFinalThreads) FinalSelectKernel(const StreamA
 //
 // One CTA per query over the query's candidate buffer (every document a tile
 // appended at or above the running bound): candidates below the final floor are
-// dropped, the K-th largest FP32 key (bit pattern of a positive score) is found by
-// two histograms in shared memory (or three radix passes of 11/10/10 bits), the documents
+// dropped; up to K, or kLargeFew, of them go straight to the sort; of more, the K-th
+// largest FP32 key (bit pattern of a positive score) is found by two histograms in
+// shared memory (or three radix passes of 11/10/10 bits), the documents
 // above it are taken whole and the ties at it by ascending id (sorted in shared
 // memory, or by a second radix select on ids when they do not fit), then the K
 // results are sorted by (score desc, id asc) with a bitonic network and the
@@ -1205,6 +1206,12 @@ constexpr int kLargeThreads = 1024;
 constexpr int kLargeMaxK = 1024;
 constexpr int kLargeEqCap = 2048;
 constexpr int kRadixBins = 4096;
+// Candidates that are sorted whole although K is below: two histograms take longer than sorting a few
+// more (K 100 on 8192 documents, 64 queries: 103 us a Search with histograms always, 98 with this at
+// K, 95 to 96 at 256; 512 threads for the kernel instead of 1024 gave nothing there and cost 15 us at
+// 8 queries of K 1000 on 1M documents).
+constexpr int kLargeFew = 256;
+static_assert(kLargeFew <= kLargeMaxK, "they fit the sorted list");
 
 struct LargeShared {
     unsigned hist[kRadixBins];
@@ -1240,8 +1247,7 @@ __device__ inline int FindBin(LargeShared &sh, int bins, unsigned need, unsigned
     if (lane == 31)
         sh.wsum[warp] = incl;
     __syncthreads();
-    for (int w = 0; w < warp; ++w)
-        incl += sh.wsum[w];
+    incl += __reduce_add_sync(kFull, lane < warp ? sh.wsum[lane] : 0u);  // the warps before this one
     const unsigned excl = incl - local;
     if (tid == kLargeThreads - 1)
         sh.total = incl;
@@ -1331,22 +1337,29 @@ __device__ unsigned RadixSelect31(LargeShared &sh, int n, const KeyOf &key_of, u
 }
 
 // Bitonic sort of p (a power of two <= 2048) entries in shared memory; `before(i, j)`
-// orders entry i ahead of entry j; `swap(i, j)` exchanges them.  Every thread calls.
+// orders entry i ahead of entry j; `swap(i, j)` exchanges them.  Every thread calls, and thread t
+// owns pair t of each step: a warp's pairs lie within its own 64 entries for strides up to 32, so
+// only the wider steps need the CTA's barrier (15 of the 55 steps of 1024 entries).
 template <class Before, class Swap>
 __device__ void BlockBitonic(int p, const Before &before, const Swap &swap)
 {
+    static_assert(kLargeMaxK <= 2 * kLargeThreads && kLargeEqCap <= 2 * kLargeThreads, "one pair per thread and step");
+    const int t = threadIdx.x;
     for (int size = 2; size <= p; size <<= 1)
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = threadIdx.x; i < p; i += kLargeThreads) {
-                const int j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    if (up ? before(j, i) : before(i, j))
-                        swap(i, j);
-                }
+            if (t < p >> 1) {
+                const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                const bool up = (i & size) == 0;
+                if (up ? before(j, i) : before(i, j))
+                    swap(i, j);
             }
-            __syncthreads();
+            const int next = stride > 1 ? stride >> 1 : size;  // the next step's stride
+            if (stride > 32 || next > 32)  // uniform
+                __syncthreads();
+            else
+                __syncwarp();
         }
+    __syncthreads();
 }
 
 // Each listed term's posting scores at ranks 64, 128, 256, 512 and 1024 (largest first; 0 past the
@@ -1469,17 +1482,20 @@ __global__ void __launch_bounds__(kLargeThreads) FinalSelectLargeKernel(const St
     // on 1M documents (889 -> 643 us a Search).
     const unsigned floor_key = max(__float_as_uint(floor), 1u);
     auto bin_of = [&](unsigned key) { return min((key - floor_key) >> 12, (unsigned)kRadixBins - 1u); };
-    for (int i = tid; i < kRadixBins; i += kLargeThreads)
-        sh.hist[i] = 0u;
-    __syncthreads();
-    ScanScores(cs, n, [&](int, float s) {
-        if (s > 0.0f && s >= floor)
-            atomicAdd(&sh.hist[bin_of(__float_as_uint(s))], 1u);
-    });
-    __syncthreads();
-    unsigned above = 0;
-    const int bin = FindBin(sh, kRadixBins, (unsigned)k, &above);
-    const unsigned total = sh.total;
+    unsigned above = 0, total = 0;
+    int bin = 0;
+    if (n > max(k, kLargeFew)) {  // uniform
+        for (int i = tid; i < kRadixBins; i += kLargeThreads)
+            sh.hist[i] = 0u;
+        __syncthreads();
+        ScanScores(cs, n, [&](int, float s) {
+            if (s > 0.0f && s >= floor)
+                atomicAdd(&sh.hist[bin_of(__float_as_uint(s))], 1u);
+        });
+        __syncthreads();
+        bin = FindBin(sh, kRadixBins, (unsigned)k, &above);
+        total = sh.total;
+    }
     unsigned kth_key = 0, need = 0;
     if (total > (unsigned)k && bin == kRadixBins - 1) {
         kth_key = RadixSelect31(sh, n, score_key, (unsigned)k, &need);
@@ -1498,14 +1514,15 @@ __global__ void __launch_bounds__(kLargeThreads) FinalSelectLargeKernel(const St
         kth_key = base + (unsigned)FindBin(sh, kRadixBins, need, &above);
         need -= above;
     }
-    // documents above the K-th key (all of them when no more than K qualify); ties at it apart
+    // documents above the K-th key (all of them when no more than K qualify, or few are there); ties
+    // at it apart
     ScanScores(cs, n, [&](int i, float s) {
         if (!(s > 0.0f && s >= floor))
             return;
         const unsigned key = __float_as_uint(s);
         if (total <= (unsigned)k || key > kth_key) {
             const unsigned at = atomicAdd(&sh.sel_count, 1u);
-            if (at < (unsigned)kLargeMaxK) {  // at most K - 1 by the radix select
+            if (at < (unsigned)kLargeMaxK) {  // at most max(K, kLargeFew); K - 1 after a select
                 sh.sel_s[at] = __uint_as_float(key);
                 sh.sel_i[at] = __ldcg(ci + i);
             }
@@ -1566,11 +1583,11 @@ __global__ void __launch_bounds__(kLargeThreads) FinalSelectLargeKernel(const St
             sh.sel_count = (unsigned)k;
     }
     __syncthreads();
-    const int c = (int)min(sh.sel_count, (unsigned)k);
+    const int taken = (int)sh.sel_count, c = min(taken, k);
     int p = 1;
-    while (p < c)
+    while (p < taken)
         p <<= 1;
-    for (int i = c + tid; i < p; i += kLargeThreads) {
+    for (int i = taken + tid; i < p; i += kLargeThreads) {
         sh.sel_s[i] = -1.0f;
         sh.sel_i[i] = INT_MAX;
     }

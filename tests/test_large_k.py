@@ -187,3 +187,25 @@ def test_large_k_from_seeds_with_ties(pkg, oracle_mod, cuda_ok, k):
             assert_same_topk(scores[start:start + kq], got[start:start + kq], ref[0].ravel(), ref[1].ravel(), f'q={q}')
             start += kq
         assert s.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_large_k_with_few_candidates(pkg, oracle_mod, cuda_ok):
+    """Candidate counts at the edges of the whole sort (K, 256) and of the sorted list (1024), with ties
+    across the K-th score, through the plain path and the safe bounds."""
+    rng = np.random.default_rng(6)
+    docs = 20_000
+    counts = [1, 33, 34, 99, 100, 101, 255, 256, 257, 258, 1023, 1024, 1025, 3000]
+    ids = [np.sort(rng.choice(docs, size=n, replace=False)).astype(np.int32) for n in counts]
+    data = [rng.choice([0.5, 0.75, 3.0], n).astype(np.float32) for n in counts]
+    indptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    ids, data = np.concatenate(ids), np.concatenate(data)
+    rows = [[t] for t in range(len(counts))] + [[0, 6], [4, 5], [7, 7], [1, 8, 2], []]
+    offsets, words = pack(rows)
+    with pkg.Bm25Session.from_csc(indptr, ids, data, docs, query_capacity=32, word_capacity=64, max_k=1024,
+                                  prune=True) as s:
+        for k in (33, 64, 100, 255, 256, 257, 1023, 1024):
+            want = oracle_mod.search(indptr, ids, data, docs, offsets, words, k)
+            assert_same_topk(*s.search((offsets, words), k), *want, f'k={k}')
+            assert_same_topk(*s.search_learned((offsets, words), k)[:2], *want, f'k={k} learned')
+        assert s.device_status() == 0
