@@ -1309,8 +1309,11 @@ class Engine {
             // (block-tile kernel, also on the plan rows); that of a batch whose largest K is above 32 runs
             // the tile-group kernel on the (query word, tile) plan: its bound rises late, and the warp-tile
             // kernel's wider first wave of claims appends far more candidates.  Tile-group against
-            // warp-tile kernel, us a Search: 50 queries at K 10 and 32 on 262,147 documents 99 / 90 to 97; 37 at
-            // K 1000 on 1M 434 / 477; 256 at K 10, 100 and 1000 on 8.8M 6180 / 7542.
+            // warp-tile kernel, us a Search, a K of 10 and 32 per query: 256 queries of 1 to 12 words on 8192
+            // documents 142 / 130, on 262,147 325 / 241, on 4.2M 2764 / 1440; 64 of 20 to 64 words on 4.2M
+            // 4389 / 2024; 129 of 256 (the rest padding) on 4.2M 1168 / 619; 1 query on 8192 66 / 55, on
+            // 262,147 63 / 56, on 4.2M 73 / 59.  K above 32: 37 queries at K 1000 on 1M 434 / 477; 256 at K 10,
+            // 100 and 1000 on 8.8M 6180 / 7542.
             const bool wt_session = plan_.kernel == BM25_KERNEL_WARP_TILE;
             const bool warp_tile = wt_session && !tau && k <= bm25k::kMaxSmallK;
             // the streaming passes after a first pass (retries, routed queries) run the warp-tile kernel
@@ -1320,10 +1323,10 @@ class Engine {
             const bool rows_only = wt_session && tau != nullptr;
             sa.rows_plan = rows_only ? 1 : 0;
             // the tile-group first pass starts from the words' seeds too (the block path writes its own
-            // bound): otherwise every claim taken before the first tiles are selected appends all it has
-            // (37 queries at K 1000 on 1M documents: 643 -> 434 us a Search; 256 mixed queries on 8.8M:
-            // 7.2 -> 6.2 ms; 50 queries at K 10 and 32 on 262,147: 156 -> 99 us)
-            sa.seed_threshold = wt_session && !tau && (kq || !warp_tile) ? 1 : 0;
+            // bound, and the warp-tile kernel takes the seeds from the word records): otherwise every claim
+            // taken before the first tiles are selected appends all it has (37 queries at K 1000 on 1M
+            // documents: 643 -> 434 us a Search; 256 mixed queries on 8.8M: 7.2 -> 6.2 ms)
+            sa.seed_threshold = wt_session && !tau && !warp_tile ? 1 : 0;
             sa.plan_rows = plan_rows_;
             sa.word_rec = word_rec_;
             sa.prefetch = 1;

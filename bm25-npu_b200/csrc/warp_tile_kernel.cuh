@@ -482,9 +482,9 @@ __global__ void __launch_bounds__(kPlanThreads) PlanRowsKernel(const StreamArgs 
         const int term = __ldg(a.words + w);
         int *out = a.plan_rows + w * a.dir_stride;
         const bool known = term >= 0 && term < a.vocab;
-        // a K per query, or a threshold to seed: the word's query is the number of q in [1, Q] with qoffsets[q] <= w (the last
-        // query starting at or before w), counted by the whole CTA at once (a malformed batch is
-        // flagged by the search kernel and fails as a whole)
+        // a K per query, or a threshold to seed: the word's query is the number of q in [1, Q] with
+        // qoffsets[q] <= w (the last query starting at or before w), counted by the whole CTA at once
+        // (a malformed batch is flagged by the search kernel and fails as a whole)
         int wq = 0;
         if ((a.kq || a.seed_threshold) && blockIdx.y == 0) {  // uniform
             for (int base = 1; base <= a.q; base += kPlanThreads)

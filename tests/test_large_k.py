@@ -209,3 +209,66 @@ def test_large_k_with_few_candidates(pkg, oracle_mod, cuda_ok):
             assert_same_topk(*s.search((offsets, words), k), *want, f'k={k}')
             assert_same_topk(*s.search_learned((offsets, words), k)[:2], *want, f'k={k} learned')
         assert s.device_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('max_k', [32, 1000])
+def test_batch_of_small_k_per_query(pkg, oracle_mod, corpus, cuda_ok, max_k):
+    """Batches whose K are all at most 32, on the default kernel: empty queries first, in the middle and
+    last, unknown words, 33 to 64 words, batches below their bucket and below the capacity, every claim
+    size, through host and device buffers."""
+    import torch
+    index, data = corpus
+    rng = np.random.default_rng(max_k)
+    df = np.diff(index.offsets)
+    common = [int(x) for x in np.argsort(-df)[:40]]
+    rows = mixed_queries(index.vocab, rng, 48, 0, 10, oov=True)
+    rows += [list(rng.integers(0, index.vocab, n)) for n in (32, 33, 63, 64)] + [common[:33], common[:1], common[:4]]
+    rows = [[]] + rows[:30] + [[], [index.vocab + 7], []] + rows[30:] + [[]]  # 60 queries: a bucket of 64, a capacity of 96
+    dev = torch.device('cuda:0')
+    with pkg.Bm25Session.from_csc(index.offsets, index.docs, data, index.num_docs, query_capacity=96,
+                                  word_capacity=2048, max_k=max_k) as s:
+        for count, tuning in ((60, {}), (60, {'claim_tiles': 2, 'tail_claims': 0}), (60, {'claim_tiles': 8}),
+                              (60, {'claim_tiles': 4, 'tail_claims': 0}), (3, {}), (1, {})):
+            s.set_tuning(**tuning)
+            part = rows[:count] if count > 3 else rows[-3:-3 + count or None]
+            offsets, words = pack([[int(x) for x in r] for r in part])
+            ks = rng.choice([1, 7, 10, 31, 32], count).astype(np.int32)
+            want_s, want_i = _by_k(oracle_mod, index, data, offsets, words, ks)
+            for _ in range(2):  # the second finds the state that the first left
+                got_s, got_i, koff = s.search_batch((offsets, words), ks)
+                assert_same_topk(got_s[None], got_i[None], want_s[None], want_i[None], f'{count} {tuning}')
+            d = [torch.from_numpy(x).to(dev) for x in (offsets, words, ks, koff[:-1].copy())]
+            d_s = torch.empty(int(koff[-1]), dtype=torch.float32, device=dev)
+            d_i = torch.empty(int(koff[-1]), dtype=torch.int32, device=dev)
+            s.search_batch_device(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), d[3].data_ptr(), count,
+                                  int(ks.max()), d_s.data_ptr(), d_i.data_ptr(), None, False,
+                                  torch.cuda.current_stream(dev).cuda_stream)
+            torch.cuda.synchronize()
+            assert s.device_status() == 0
+            assert_same_topk(d_s.cpu().numpy()[None], d_i.cpu().numpy()[None], want_s[None], want_i[None],
+                             f'device {count} {tuning}')
+
+
+@pytest.mark.gpu
+def test_batch_of_small_k_with_ties_at_the_seed(pkg, oracle_mod, cuda_ok):
+    """A K per query up to 32 where the word's K-th posting score, the bound that its query starts from,
+    is tied past rank K, and where a list holds exactly K, K - 1 and one posting."""
+    rng = np.random.default_rng(12)
+    docs = 150_001
+    counts = [docs // 3, 32, 31, 10, 9, 1, 5000]
+    ids = [np.sort(rng.choice(docs, size=n, replace=False)).astype(np.int32) for n in counts]
+    data = [np.full(n, 1.0 + i, np.float32) for i, n in enumerate(counts)]
+    data[-1] = np.exp2(rng.uniform(-20, 20, counts[-1])).astype(np.float32)
+    indptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    ids, data = np.concatenate(ids), np.concatenate(data)
+    rows = [[0], [1], [2], [3], [4], [5], [6], [0, 1], [0, 0], [6, 0], [4, 3, 2, 1], []]
+    offsets, words = pack(rows)
+    with pkg.Bm25Session.from_csc(indptr, ids, data, docs, query_capacity=32, word_capacity=64, max_k=32) as s:
+        for first in range(3):
+            ks = np.resize(np.array([32, 10, 1][first:] + [31, 9], np.int32), len(rows))
+            got_s, got_i, koff = s.search_batch((offsets, words), ks)
+            for q, k in enumerate(ks):
+                ref = oracle_mod.search(indptr, ids, data, docs, *pack([rows[q]]), int(k))
+                assert_same_topk(got_s[koff[q]:koff[q] + k], got_i[koff[q]:koff[q] + k], ref[0].ravel(),
+                                 ref[1].ravel(), f'q={q} k={k}')
