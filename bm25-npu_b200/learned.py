@@ -106,12 +106,14 @@ def train(features, targets, *, steps=3000, batch=4096, lr=2e-3, over_weight=4.0
     import torch
     lib = n.engine_library()
     dev = torch.device(device)
-    x = torch.from_numpy(np.ascontiguousarray(features, dtype=np.float32)).to(dev)
-    t = torch.from_numpy(np.ascontiguousarray(targets, dtype=np.float32)).to(dev)
+    x = torch.from_numpy(np.ascontiguousarray(features, dtype=np.float32))
+    t = torch.from_numpy(np.ascontiguousarray(targets, dtype=np.float32))
     count = x.shape[0]
     batch = min(batch, count)
+    # the backward kernel reads 32 features and one target of every row that is drawn
     if x.numel() != count * FEATURES or t.numel() != t.shape[0] or t.shape[0] < count:
         raise ValueError('train: features [N, 32] and one target per row expected')
+    x, t = x.to(dev), t.to(dev)
     p = torch.from_numpy(init_params(seed, float(np.mean(targets)))).to(dev)
     m = torch.zeros_like(p)
     v = torch.zeros_like(p)

@@ -181,3 +181,28 @@ def test_overlapped_training_steps_see_each_update(pkg, cuda_ok, batch):
                                     losses.data_ptr(), None) == 0
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got + [losses], want + [loss]))
+
+
+@pytest.mark.parametrize('features,targets', [((50, 31), (50,)), ((50, 33), (50,)), ((50, 32), (49,)),
+                                              ((50, 32), (50, 2)), ((64,), (64,))])
+def test_train_refuses_features_the_kernel_would_misread(pkg, features, targets):
+    """Rows of another width than 32, or fewer targets than rows, are refused before the device is used."""
+    with pytest.raises(ValueError, match='features'):
+        pkg.learned.train(np.zeros(features, np.float32), np.zeros(targets, np.float32), steps=1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('features,targets', [((40, 32), (40,)), ((40, 32), (40, 1)), ((40, 4, 8), (40,)),
+                                              ((40, 32), (45,))])
+def test_train_accepts_whole_rows(pkg, cuda_ok, features, targets):
+    """Any shape that holds 32 features and one target per row trains the same model."""
+    rng = np.random.default_rng(1)
+    x, t = rng.normal(size=(40, 32)).astype(np.float32), rng.normal(size=40).astype(np.float32)
+    want, want_loss = pkg.learned.train(x, t, steps=9, batch=16)
+    y = np.full(int(np.prod(targets)), t.mean(), np.float32)
+    y[:40] = t
+    got, loss = pkg.learned.train(x.reshape(features), y.reshape(targets), steps=9, batch=16)
+    if y.size == 40:
+        assert np.array_equal(got, want) and np.array_equal(loss, want_loss)
+    else:  # the targets' mean starts the bias: equal to rounding
+        assert np.allclose(got, want, atol=1e-4) and np.allclose(loss, want_loss, rtol=1e-3)
