@@ -181,6 +181,13 @@ def write_bm25s_dir(indptr, indices, data, num_docs, path, k1=1.5, b=0.75):
                                                        indent=4))
 
 
+def _trimmed(a, k):
+    """a[:k]: a view, which keeps all of a, or a copy when less than two thirds of a are used.  Documents
+    of 60 to 80 Zipf tokens have 0.72 to 0.82 postings per token; copying both arrays then makes a build
+    of 200,003 documents 42 ms instead of 25.5."""
+    return a[:k] if 3 * k >= 2 * a.size else a[:k].copy()
+
+
 def build_index(doc_offsets, tokens, vocab, k1=1.2, b=0.75, device_id=0):
     """The reference's lazy index from documents given as token ids, built on the GPU
     (bm25_build_index: key sort and run-length counts on the device, idf and norms in double
@@ -205,6 +212,5 @@ def build_index(doc_offsets, tokens, vocab, k1=1.2, b=0.75, device_id=0):
         lib.bm25_build_last_error(buf, len(buf))
         raise ValueError(f'index build failed ({status}): {buf.value.decode()}')
     k = m.value
-    # the arrays are as long as the tokens; the pages past the postings were never touched
-    return LazyIndex(offsets, docs[:k], tf[:k], norm, idf,
+    return LazyIndex(offsets, _trimmed(docs, k), _trimmed(tf, k), norm, idf,
                      np.diff(doc_offsets).astype(np.int32))

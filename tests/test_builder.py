@@ -68,3 +68,27 @@ def test_gpu_builder_matches_reference_and_restatement(pkg, oracle_mod, golden, 
     bad[17] = 70_000
     with pytest.raises(ValueError):
         pkg.build_index(doc_offsets, bad, 70_000)
+
+
+def _kept(a):
+    """Elements that stay allocated for the array a."""
+    return a.size if a.base is None else a.base.size
+
+
+@pytest.mark.parametrize('k,size', [(0, 1), (1, 1), (2, 3), (65, 100), (66, 100), (67, 100), (100, 100)])
+def test_trimmed_keeps_at_most_half_again(pkg, k, size):
+    a = np.arange(size, dtype=np.int32)
+    t = pkg.corpus._trimmed(a, k)
+    assert np.array_equal(t, a[:k]) and _kept(t) <= k + k // 2
+
+
+@pytest.mark.gpu
+def test_index_of_repeated_terms_keeps_no_token_arrays(pkg, cuda_ok):
+    """20,000 documents of 50 tokens out of 8 terms: 8 postings a document, not 50."""
+    from oracle import build_oracle
+    doc_offsets = np.arange(20_001, dtype=np.int64) * 50
+    tokens = np.random.default_rng(3).integers(0, 8, 1_000_000).astype(np.int32)
+    idx = pkg.build_index(doc_offsets, tokens, 8)
+    assert _kept(idx.docs) <= 1.5 * idx.docs.size and _kept(idx.tf) <= 1.5 * idx.tf.size
+    _same_index((idx.offsets, idx.docs, idx.tf, idx.norm, idx.idf),
+                dict(zip(('offsets', 'docs', 'tf', 'norm', 'idf'), build_oracle.build(doc_offsets, tokens, 8))), 'repeats')
