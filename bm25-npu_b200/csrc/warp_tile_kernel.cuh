@@ -290,7 +290,9 @@ __global__ void __launch_bounds__(kWtThreads, 3) WarpTileKernel(const StreamArgs
             bad |= kStatusBadQuery;
             nw = 0;
         }
-        if (nw == 0) {  // uniform: nothing to scan (a batch is padded to its bucket with empty queries)
+        // uniform: nothing to scan.  Batches are padded to their bucket with empty queries; a Search of one
+        // K is not, and goes without the branch (with it 162 queries of K 32 on 1.6M documents 286 -> 290 us)
+        if (!kLean && nw == 0) {
             if (lane == 0)
                 sh.counters[warp][0] += 1u;
             continue;
