@@ -425,7 +425,7 @@ def learned_leg(pkg, args, spec, index, session, sets, want, flush, stream, dev_
     out['learned']['model'] = {'train_queries': model.report['train_queries'], 'train_s': train_s,
                                'margin': model.margin, 'val_fallback': model.report['val_fallback'],
                                'first_loss': model.report['first_loss'], 'last_loss': model.report['last_loss'],
-                               'trained_with': 'bm25_mlp_gradient + bm25_mlp_adam (engine kernels)'}
+                               'trained_with': 'bm25_mlp_train_steps (engine kernels)'}
     return out
 
 

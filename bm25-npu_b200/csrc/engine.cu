@@ -1359,26 +1359,35 @@ class Engine {
             const long long claims = (long long)q * ((plan_.tiles + bm25k::kWgWarps - 1) / bm25k::kWgWarps);
             const int wg_grid = (int)std::max<long long>(1, std::min<long long>(tg_grid_, claims));
             const int ct = tuning_.claim_tiles;
-            // one warp per tile while the chip has them (the claims below are then all single tiles): a grid
-            // of one warp per claim of ct tiles left most SMs idle and a chain of tiles to each warp on
-            // small work, where a batch of K <= 32 took longer than on the tile-group kernel (1 query on
-            // 262,147 documents 62 us against 60, 256 on 8192 162 against 147; 57 and 140 with this grid)
-            const long long wt_tiles = (long long)q * plan_.tiles;
-            const int wt_grid = (int)std::max<long long>(
-                1, std::min<long long>(plan_.grid, (wt_tiles + bm25k::kWtWarps - 1) / bm25k::kWtWarps));
-            {
-                // single-tile claims for the last tiles: tail_claims per warp of the launch
-                const long long tail = ((long long)tuning_.tail_claims * wt_grid * bm25k::kWtWarps + q - 1) / q;
-                sa.wt_bulk = (int)std::max<long long>(0, (plan_.tiles - tail) / ct);
-            }
+            // Warp-tile launches: one warp per unit while the chip has them, and single-tile claims for the
+            // last tiles (tail_claims per warp of the launch).  A first pass counts tiles (its claims are then
+            // all single ones on small work): a warp per claim of ct tiles left most SMs idle and a chain of
+            // tiles to each warp, where a batch of K <= 32 took longer than on the tile-group kernel (1 query
+            // on 262,147 documents 62 us against 60, 256 on 8192 162 against 147; 57 and 140 with this grid).
+            // A retry pass counts claims, as its list is empty as a rule and a wider launch takes longer to
+            // end (1 query on 262,147 documents, 32 CTAs instead of 8: 2.9 us against 2.7).
+            const long long wt_tiles = (long long)q * plan_.tiles, wt_claims = (long long)q * ((plan_.tiles + ct - 1) / ct);
+            auto wt_grid = [&](long long units) {
+                return (int)std::max<long long>(
+                    1, std::min<long long>(plan_.grid, (units + bm25k::kWtWarps - 1) / bm25k::kWtWarps));
+            };
+            auto wt_bulk = [&](int grid) {
+                const long long tail = ((long long)tuning_.tail_claims * grid * bm25k::kWtWarps + q - 1) / q;
+                return (int)std::max<long long>(0, (plan_.tiles - tail) / ct);
+            };
+            const int wt_first = wt_grid(wt_tiles), wt_retry = wt_grid(wt_claims);
+            sa.wt_bulk = wt_bulk(wt_first);
             auto tile_group = [&](const bm25k::StreamArgs &args) {
                 const bool lean = !args.retry && !args.kq && k <= bm25k::kMaxSmallK;
                 if (warp_tile || (wt_streams && args.retry)) {
-                    if (!args.retry)  // right after the plan rows: set up while they are built
-                        LaunchOverlapped(lean ? WarpTileFor<true>(ct) : WarpTileFor<false>(ct), wt_grid,
+                    if (!args.retry) {  // right after the plan rows: set up while they are built
+                        LaunchOverlapped(lean ? WarpTileFor<true>(ct) : WarpTileFor<false>(ct), wt_first,
                                          bm25k::kWtThreads, smem_bytes_, s, args);
-                    else
-                        WarpTileFor<false>(ct)<<<wt_grid, bm25k::kWtThreads, smem_bytes_, s>>>(args);
+                    } else {
+                        bm25k::StreamArgs again = args;
+                        again.wt_bulk = wt_bulk(wt_retry);
+                        WarpTileFor<false>(ct)<<<wt_retry, bm25k::kWtThreads, smem_bytes_, s>>>(again);
+                    }
                 } else if (plan_.tile_docs == 2048) {
                     if (lean)
                         bm25k::TileGroupKernel<2048, true><<<wg_grid, bm25k::kWgThreads, tg_smem_, s>>>(args);
