@@ -1211,7 +1211,7 @@ constexpr int kRadixBins = 4096;
 // K, 95 to 96 at 256; 512 threads for the kernel instead of 1024 gave nothing there and cost 15 us at
 // 8 queries of K 1000 on 1M documents).
 constexpr int kLargeFew = 256;
-static_assert(kLargeFew <= kLargeMaxK, "they fit the sorted list");
+static_assert(kLargeFew <= kLargeMaxK && kLargeMaxK <= kLargeThreads, "they fit the sorted list, one per thread");
 
 struct LargeShared {
     unsigned hist[kRadixBins];
@@ -1473,18 +1473,26 @@ __global__ void __launch_bounds__(kLargeThreads) FinalSelectLargeKernel(const St
         *key = __float_as_uint(s);
         return s > 0.0f && s >= floor;
     };
-    // The K-th key by two histograms of 4096 bins: of the keys' distance from the floor's in steps of
-    // 4096 (two octaves of scores; the last bin takes the rest), then of the keys in the bin that
-    // holds it.  The bits of the keys themselves would put nearly all candidates, which lie within an
-    // octave or two, into a few bins whose atomics queue up.  A K-th key in the last bin (a floor far
-    // below it) falls back to the radix passes.  Three passes over the candidates in 128-bit loads by
-    // 1024 threads, where five in single loads by 512 took 430 us of a Search of 37 queries at K 1000
-    // on 1M documents (889 -> 643 us a Search).
-    const unsigned floor_key = max(__float_as_uint(floor), 1u);
-    auto bin_of = [&](unsigned key) { return min((key - floor_key) >> 12, (unsigned)kRadixBins - 1u); };
-    unsigned above = 0, total = 0;
-    int bin = 0;
-    if (n > max(k, kLargeFew)) {  // uniform
+    unsigned total = 0, kth_key = 0, need = 0;
+    if (n <= max(k, kLargeFew)) {  // uniform: every candidate at or above the floor, one per thread
+        const float s = tid < n ? __ldcg(cs + tid) : 0.0f;
+        const int id = tid < n ? __ldcg(ci + tid) : 0;
+        if (s > 0.0f && s >= floor) {
+            const unsigned at = atomicAdd(&sh.sel_count, 1u);
+            sh.sel_s[at] = s;
+            sh.sel_i[at] = id;
+        }
+    } else {
+        // The K-th key by two histograms of 4096 bins: of the keys' distance from the floor's in steps of
+        // 4096 (two octaves of scores; the last bin takes the rest), then of the keys in the bin that
+        // holds it.  The bits of the keys themselves would put nearly all candidates, which lie within an
+        // octave or two, into a few bins whose atomics queue up.  A K-th key in the last bin (a floor far
+        // below it) falls back to the radix passes.  Three passes over the candidates in 128-bit loads by
+        // 1024 threads, where five in single loads by 512 took 430 us of a Search of 37 queries at K 1000
+        // on 1M documents (889 -> 643 us a Search).
+        const unsigned floor_key = max(__float_as_uint(floor), 1u);
+        auto bin_of = [&](unsigned key) { return min((key - floor_key) >> 12, (unsigned)kRadixBins - 1u); };
+        unsigned above = 0;
         for (int i = tid; i < kRadixBins; i += kLargeThreads)
             sh.hist[i] = 0u;
         __syncthreads();
@@ -1493,45 +1501,43 @@ __global__ void __launch_bounds__(kLargeThreads) FinalSelectLargeKernel(const St
                 atomicAdd(&sh.hist[bin_of(__float_as_uint(s))], 1u);
         });
         __syncthreads();
-        bin = FindBin(sh, kRadixBins, (unsigned)k, &above);
+        const int bin = FindBin(sh, kRadixBins, (unsigned)k, &above);
         total = sh.total;
-    }
-    unsigned kth_key = 0, need = 0;
-    if (total > (unsigned)k && bin == kRadixBins - 1) {
-        kth_key = RadixSelect31(sh, n, score_key, (unsigned)k, &need);
-    } else if (total > (unsigned)k) {
-        const unsigned base = floor_key + ((unsigned)bin << 12);
-        for (int i = tid; i < kRadixBins; i += kLargeThreads)
-            sh.hist[i] = 0u;
-        __syncthreads();
-        ScanScores(cs, n, [&](int, float s) {
-            const unsigned key = __float_as_uint(s);
-            if (s > 0.0f && s >= floor && key - base < (unsigned)kRadixBins)
-                atomicAdd(&sh.hist[key - base], 1u);
-        });
-        __syncthreads();
-        need = (unsigned)k - above;
-        kth_key = base + (unsigned)FindBin(sh, kRadixBins, need, &above);
-        need -= above;
-    }
-    // documents above the K-th key (all of them when no more than K qualify, or few are there); ties
-    // at it apart
-    ScanScores(cs, n, [&](int i, float s) {
-        if (!(s > 0.0f && s >= floor))
-            return;
-        const unsigned key = __float_as_uint(s);
-        if (total <= (unsigned)k || key > kth_key) {
-            const unsigned at = atomicAdd(&sh.sel_count, 1u);
-            if (at < (unsigned)kLargeMaxK) {  // at most max(K, kLargeFew); K - 1 after a select
-                sh.sel_s[at] = __uint_as_float(key);
-                sh.sel_i[at] = __ldcg(ci + i);
-            }
-        } else if (key == kth_key) {
-            const unsigned at = atomicAdd(&sh.eq_count, 1u);
-            if (at < (unsigned)kLargeEqCap)
-                sh.eq[at] = __ldcg(ci + i);
+        if (total > (unsigned)k && bin == kRadixBins - 1) {
+            kth_key = RadixSelect31(sh, n, score_key, (unsigned)k, &need);
+        } else if (total > (unsigned)k) {
+            const unsigned base = floor_key + ((unsigned)bin << 12);
+            for (int i = tid; i < kRadixBins; i += kLargeThreads)
+                sh.hist[i] = 0u;
+            __syncthreads();
+            ScanScores(cs, n, [&](int, float s) {
+                const unsigned key = __float_as_uint(s);
+                if (s > 0.0f && s >= floor && key - base < (unsigned)kRadixBins)
+                    atomicAdd(&sh.hist[key - base], 1u);
+            });
+            __syncthreads();
+            need = (unsigned)k - above;
+            kth_key = base + (unsigned)FindBin(sh, kRadixBins, need, &above);
+            need -= above;
         }
-    });
+        // documents above the K-th key (all of them when no more than K qualify); ties at it apart
+        ScanScores(cs, n, [&](int i, float s) {
+            if (!(s > 0.0f && s >= floor))
+                return;
+            const unsigned key = __float_as_uint(s);
+            if (total <= (unsigned)k || key > kth_key) {
+                const unsigned at = atomicAdd(&sh.sel_count, 1u);
+                if (at < (unsigned)kLargeMaxK) {  // at most K - 1 by the select
+                    sh.sel_s[at] = __uint_as_float(key);
+                    sh.sel_i[at] = __ldcg(ci + i);
+                }
+            } else if (key == kth_key) {
+                const unsigned at = atomicAdd(&sh.eq_count, 1u);
+                if (at < (unsigned)kLargeEqCap)
+                    sh.eq[at] = __ldcg(ci + i);
+            }
+        });
+    }
     __syncthreads();
     if (total > (unsigned)k) {
         const unsigned eqn = sh.eq_count;
