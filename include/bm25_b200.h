@@ -238,7 +238,8 @@ int bm25_search_learned_device(bm25_handle *handle, const int64_t *qoffsets, con
  * Search counters summed over Searches since the last reset (waits for the
  * handle's work), out[7]: tile-group kernel -- [0] claims (query x 8-tile
  * groups), [1] tiles scanned, [2] postings copied from HBM into the staging
- * rings; block-max pruned pass -- [3] tiles scored, [4] 128-document blocks
+ * rings; warp-tile kernel -- the same of its own claims (an empty query of a
+ * batch with a K per query scans no tiles) and postings read; block-max pruned pass -- [3] tiles scored, [4] 128-document blocks
  * kept, [5] postings read, [6] queries streamed instead (prune_route).
  */
 int bm25_search_stats(bm25_handle *handle, uint64_t *out, int32_t reset);
